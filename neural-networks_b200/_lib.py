@@ -117,7 +117,9 @@ def check(rc, what):
     raise XlstmError("%s failed (%d): %s" % (what, rc, msg))
 
 
-# The C++ host path over the same library (built beside it); like the library itself, not optional.
+# The C++ host path over the same library (built beside it); like the library itself, not optional. It links torch's Python
+# library, which has to be initialised by torch itself: loaded first, it crashes the interpreter when torch is imported later.
+import torch  # noqa: E402, F401
 from . import _host as host  # noqa: E402
 
 host.init(check, XlstmError)
