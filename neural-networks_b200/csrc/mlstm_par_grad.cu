@@ -86,10 +86,10 @@ __global__ void __launch_bounds__(1024) par_gate_grad(const GgArgs p) {
         const bf16* Ce = p.recC + ((size_t)bh * (p.NC + 1) + p.NC) * DD;
         float acc = 0.f;
         for (size_t i = (size_t)tid * 4; i < DD; i += 4096) {
-            const float4 x = *reinterpret_cast<const float4*>(p.cdC + bh * DD + i);
+            const float* x = p.cdC + bh * DD + i;  // the caller's: aligned to a float and no more
             const uint2 c = *reinterpret_cast<const uint2*>(Ce + i);
             const float2 lo = unpack_bf16(c.x), hi = unpack_bf16(c.y);
-            acc += x.x * lo.x + x.y * lo.y + x.z * hi.x + x.w * hi.y;
+            acc += x[0] * lo.x + x[1] * lo.y + x[2] * hi.x + x[3] * hi.y;
         }
         if (tid < p.D) acc += p.cdn[(size_t)bh * p.D + tid] * p.recn[((size_t)bh * (p.NC + 1) + p.NC) * p.D + tid];
         run = block_sum(acc, red);
@@ -509,7 +509,7 @@ int mlstm_par_bw_launch(cudaStream_t st, const MlstmBwArgs& a, const float* carr
         return XLSTM_ERR_WORKSPACE;
     }
     if (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.ytil | (uintptr_t)a.dytil | (uintptr_t)a.dq | (uintptr_t)a.dk |
-         (uintptr_t)a.dv | (uintptr_t)saved | (uintptr_t)workspace) & 15) {
+         (uintptr_t)a.dv | (uintptr_t)a.odC | (uintptr_t)saved | (uintptr_t)workspace) & 15) {
         set_error("mlstm_bw (tensor-core path): tensors must be 16-byte aligned");
         return XLSTM_ERR_ARG;
     }

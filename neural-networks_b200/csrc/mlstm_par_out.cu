@@ -279,7 +279,7 @@ int mlstm_par_fw_launch(cudaStream_t st, const MlstmFwArgs& a, void* saved, void
         set_error("mlstm_fw: workspace of %zu B is smaller than the %zu B required", workspace_bytes, need);
         return XLSTM_ERR_WORKSPACE;
     }
-    if (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.ytil | (uintptr_t)saved | (uintptr_t)workspace) & 15) {
+    if (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.ytil | (uintptr_t)a.oC | (uintptr_t)saved | (uintptr_t)workspace) & 15) {
         set_error("mlstm_fw (tensor-core path): tensors must be 16-byte aligned");
         return XLSTM_ERR_ARG;
     }

@@ -303,10 +303,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
                 float v[32];
                 if (i == 0) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const float4 x = p.c0 ? *reinterpret_cast<const float4*>(p.c0 + crow + c * 32 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
-                    }
+                    for (int j = 0; j < 32; ++j) v[j] = p.c0 ? p.c0[crow + c * 32 + j] : 0.f;  // once a call; a caller's state may start at any float
                 } else {
                     tmem_ld32(t0 + c * 32, v);
                     tmem_ld_wait();

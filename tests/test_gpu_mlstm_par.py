@@ -71,3 +71,32 @@ def test_recomputed_states_leave_the_gradients_bit_identical():
     b = _run((2, 2, 400, 128), torch.float32, 72, True, False)[3]
     for x, y in zip(a[:5] + a[5], b[:5] + b[5]):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 385, 128), (1, 1, 65, 256)])
+def test_states_that_start_at_any_float_are_read(shape):
+    """A state cut out of a larger array starts where that array left off: on four bytes, not on sixteen."""
+    from gpu_util import ops, xl, dev, mlstm_inputs
+    B, H, T, d = shape
+    q, k, v, ig, fg, dy = mlstm_inputs(B, H, T, d, d, seed=74, bf16=True)
+    r = np.random.default_rng(75)
+    f = lambda *s: dev(r.standard_normal(s))
+    carry, dst = (f(B * H, d, d), f(B * H, d), f(B * H)), (f(B * H, d, d), f(B * H, d))
+
+    def shifted(x):
+        out = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape)
+        out.copy_(x)
+        assert out.data_ptr() % 16 == 4
+        return out
+
+    bf = torch.bfloat16
+    st = ops.MlstmShape(B, H, T, d, d, 64, bf, torch.float32)
+    args = (dev(q, bf), dev(k, bf), dev(v, bf), dev(ig), dev(fg))
+    res = []
+    for c, ds in ((carry, dst), (tuple(map(shifted, carry)), tuple(map(shifted, dst)))):
+        fused = ops.mlstm_fused_fw(*args, st, carry_in=c)
+        g = ops.mlstm_fused_bw(fused, *args, dev(dy), st, carry_in=c, dstate_in=ds)
+        torch.cuda.synchronize()
+        res.append((fused.ytil, *fused.state, *g[:5], *g[5]))
+    assert xl._lib.lib.xlstm_device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(*res))
