@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(1024) ce_row_cta(const float* __restrict__ log
         const float is = 1.f / gsum;
         const uint32_t tg = targets[r];
         if (threadIdx.x == 0) {
-            float zt = CACHE ? sr[tg] : capped<CAP>(z[tg], cap, icap);
-            float pt = expf(zt - gmx) * is;
+            float pt = 0.f;  // a target that is no symbol has none
+            if (tg < (uint32_t)C) pt = expf((CACHE ? sr[tg] : capped<CAP>(z[tg], cap, icap)) - gmx) * is;
             loss -= logf(fmaxf(pt, 1e-30f));
         }
         if (!CACHE) __syncthreads();  // dlogits may alias logits: read z[target] before anyone overwrites it
@@ -195,7 +195,8 @@ __device__ __forceinline__ float narrow_row(const float* z, float* d, bool live,
     const float k1 = 2.f * icap * 1.4426950408889634f, k2 = (CAP ? cap : 1.f) * 1.4426950408889634f;
     auto squash = [&](float x) { return CAP ? 1.f - __fdividef(2.f, 1.f + ex2(x * k1)) : x; };
     float v[VPL], e[VPL], mx = -INFINITY, sum = 0.f;
-    const float zt = squash(z[tg]);
+    const bool any = tg < (uint32_t)C;  // a target that is no symbol: nothing is read or written for it, its probability is 0
+    const float zt = any ? squash(z[tg]) : 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
         const int j = i * 32 + lane;
@@ -220,8 +221,8 @@ __device__ __forceinline__ float narrow_row(const float* z, float* d, bool live,
         if (i < FULL || j < C) d[j] = e[i] * gs * (CAP ? fmaf(-v[i], v[i], 1.f) : 1.f);
     }
     __syncwarp();
-    const float pt = ex2(fmaf(zt, k2, -mk)) * is;
-    if (lane == 0) d[tg] = (pt - 1.f) * inv * (CAP ? fmaf(-zt, zt, 1.f) : 1.f);
+    const float pt = any ? ex2(fmaf(zt, k2, -mk)) * is : 0.f;
+    if (any && lane == 0) d[tg] = (pt - 1.f) * inv * (CAP ? fmaf(-zt, zt, 1.f) : 1.f);
     return lane == 0 ? -logf(fmaxf(pt, 1e-30f)) : 0.f;
 }
 

@@ -35,3 +35,39 @@ def test_cross_entropy_rows_of_any_width(rows, C, cap, masked, shift):
         assert ops.lib.xlstm_device_status() == 0
         assert abs(loss.item() - 1.0 - want.item()) <= 1e-5 * max(1.0, abs(want.item()))
         assert float((out.double() - x.grad).abs().max()) <= 1e-5 * max(float(x.grad.abs().max()), 1e-30)
+
+
+@pytest.mark.parametrize("rows,C,cap,shift", [(40, 61, 0.0, 0), (40, 257, 30.0, 0), (33, 1024, 0.0, 0), (20, 300, 30.0, 1), (9, 5001, 30.0, 0), (5, 60001, 0.0, 0)])
+def test_a_target_that_is_no_symbol_touches_nothing(rows, C, cap, shift):
+    """Such a row has the gradient of its softmax alone and the loss of a probability at its floor; the rows beside it, and what lies
+    behind the array, are as without it."""
+    import math
+    from gpu_util import ops
+    g = torch.Generator(device="cuda").manual_seed(C)
+    buf = torch.randn(rows * C + 4, device="cuda", generator=g) * 3.0
+    z = buf[shift:shift + rows * C].view(rows, C)
+    t = torch.randint(0, C, (rows,), device="cuda", generator=g, dtype=torch.int32)
+    bad = {1: C, 2: C + 7, 3: -1, rows - 1: 0x7fffffff}
+    for r, v in bad.items():
+        t[r] = v
+    live = torch.ones(rows, dtype=torch.bool, device="cuda")
+    live[list(bad)] = False
+    x = z.double()
+    y = cap * torch.tanh(x / cap) if cap else x
+    p = torch.softmax(y, 1)
+    one = torch.zeros_like(p)
+    one[live, t[live].long()] = 1.0
+    inv = 1.0 / rows
+    want = (p - one) * inv * ((1 - (y / cap) ** 2) if cap else 1.0)
+    loss_want = ((-(p * one).sum(1)[live].log()).sum() - len(bad) * math.log(1e-30)) * inv
+    out = torch.full((rows * C + 4,), 7.0, device="cuda")
+    d, loss = out[shift:shift + rows * C].view(rows, C), torch.zeros(1, device="cuda")
+    if cap:
+        ops.softcap_cross_entropy(z, t, d, loss, cap, inv=inv)
+    else:
+        ops.softmax_cross_entropy(z, t, d, loss, inv=inv)
+    torch.cuda.synchronize()
+    assert ops.lib.xlstm_device_status() == 0
+    assert float((d.double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+    assert abs(loss.item() - float(loss_want)) <= 1e-5 * float(loss_want)
+    assert bool((out[:shift] == 7.0).all()) and bool((out[shift + rows * C:] == 7.0).all())
