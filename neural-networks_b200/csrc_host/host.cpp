@@ -189,17 +189,17 @@ static void embedding_scatter_add(const Tensor& table_g, const Tensor& ids, cons
 
 // ---- projections: Y = X W + b --------------------------------------------------------------------------------------------------------
 // mode 0: fp32 result with the bias; 1: the product alone, fp32; 2: residual + the product + bias (the seed is one pass, the product
-// accumulates into it); 3: scale * (x W + b) rounded once to bf16 (`bb`: the bias as bf16); 4: the product alone as bf16.
-static Tensor linear_fw(const Tensor& x, const Tensor& w, const Tensor& b, const OptT& bb, int mode, const OptT& residual, double scale) {
+// accumulates into it); 3: scale * (x W + b) rounded once to bf16; 4: the product alone as bf16.
+static Tensor linear_fw(const Tensor& x, const Tensor& w, const Tensor& b, int mode, const OptT& residual, double scale) {
     Below guard;
     const bool bf = w.scalar_type() == at::kBFloat16;
     if (mode == 4) return at::mm(x, w);
     if (mode == 3) {
-        if (scale == 1.0) return at::addmm(*bb, x, w);
+        // the bias in the operand type, from the fp32 one at every call: a program may have written it since the last
         // with a factor on the bias too, the library spreads it over the whole output first and reads that back (32768 x 2048: 176 us); a power
         // of two can go into the bias beforehand without changing a bit
         int e;
-        if (std::frexp(scale, &e) != 0.5) return at::addmm(*bb, x, w, scale, scale);
+        if (scale == 1.0 || std::frexp(scale, &e) != 0.5) return at::addmm(b.to(at::kBFloat16), x, w, scale, scale);
         Tensor sb = fresh(b.sizes(), at::kBFloat16, b);
         at::mul_out(sb, b, at::scalar_tensor(scale, at::kDouble));
         return at::addmm(sb, x, w, 1, scale);

@@ -80,7 +80,7 @@ class Linear:
     def __init__(self, w, b, decay=True, bf16=False):
         self.bf16 = bf16
         self.w = Param(w, decay, shadow=bf16)
-        self.b = Param(b, False, shadow=bf16)  # the narrowed epilogues add it in the operand type
+        self.b = Param(b, False)
 
     def forward(self, x, bias=True, residual=None, narrow=False, scale=1.0):
         """x: fp32, or already narrowed to bf16 by a caller that feeds several projections from it.
@@ -92,7 +92,7 @@ class Linear:
         narrow = narrow and self.bf16
         assert scale == 1.0 or (narrow and bias), "scale is folded only into the narrowed epilogue"
         mode = (3 if bias else 4) if narrow else 2 if residual is not None else 0 if bias else 1
-        return ops.linear_forward(self.x, self.w.wb if self.bf16 else self.w.w, self.b.w, self.b.wb, mode, residual, scale)
+        return ops.linear_forward(self.x, self.w.wb if self.bf16 else self.w.w, self.b.w, mode, residual, scale)
 
     def backward(self, dy, need_dx=True, accum=None, scale=1.0, narrow_dx=False):
         """Accumulates dW, db; returns dx, added into `accum` (inside the GEMM, beta = 1) when one is given.
