@@ -240,14 +240,21 @@ static OptT linear_bw(const Tensor& dy_, const Tensor& x, const Tensor& w, const
         at::addmm_out(a, a, dy, wt, at::kFloat, 1, alpha);
         return a;
     }
-    // fp32: the scale rides in the products' alpha as well
+    // fp32: the scale rides in the products' alpha as well. The kernels take rows that lie one behind the other; gradients of any other
+    // strides (a transposed or expanded one), and none at all, go through the library.
     const int64_t rows = x.size(0), k = x.size(1), n = dy_.size(1);
-    if (x.is_contiguous() && rows * k * n <= kOwnGradWork) {
+    const bool plain = rows > 0 && dy_.is_contiguous();
+    if (plain && x.is_contiguous() && rows * k * n <= kOwnGradWork) {
         const size_t wsb = xlstm_linear_grad_f32_workspace_bytes((int)rows, (int)k, (int)n);
         Tensor ws = scratch(wsb, x);
         check(xlstm_linear_grad_f32(stream(), fptr(x), fptr(dy_), fptr(wg), fptr(bg), (int)rows, (int)k, (int)n, (float)scale, ptr(ws), wsb), "linear_grad");
     } else {
-        colsum_narrow(dy_, bg, (float)scale, false);
+        if (plain) {
+            colsum_narrow(dy_, bg, (float)scale, false);
+        } else {
+            Tensor b = bg;
+            b.add_(dy_.sum(0), scale);
+        }
         Tensor g = wg;
         g.addmm_(x.t(), dy_, 1, scale);
     }

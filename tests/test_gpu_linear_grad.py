@@ -21,3 +21,30 @@ def test_linear_gradients(rows, k, n):
     assert rc == 0
     for got, want in ((dw, want_w), (db, want_b)):
         assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
+
+
+@pytest.mark.parametrize("kind", ["transposed", "expanded", "sliced", "strided input", "no rows"])
+def test_a_projection_takes_gradients_of_any_strides(kind):
+    """The fp32 projection's backward on rows that do not lie one behind the other, and on none: as on their copies."""
+    import importlib
+    layers = importlib.import_module("neural-networks_b200.layers")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    rows, k, n = (0 if kind == "no rows" else 96), 40, 24
+    w, b, x, dy = r(k, n), r(n), r(rows, k), r(rows, n)
+    if kind == "transposed":
+        dy = r(n, rows).t()
+    elif kind == "expanded":
+        dy = r(1, n).expand(rows, n)
+    elif kind == "sliced":
+        dy = r(rows, 2 * n)[:, n:]
+    elif kind == "strided input":
+        x, dy = r(k, rows).t(), r(n, rows).t()
+    lin = layers.Linear(w, b)
+    lin.forward(x)
+    dx = lin.backward(dy, scale=0.5)
+    ref = 0.5 * dy.double()
+    for got, want in ((dx, ref @ w.double().t()), (lin.w.g, x.double().t() @ ref), (lin.b.g, ref.sum(0))):
+        assert got.shape == want.shape
+        if want.numel():
+            assert float((got.double() - want).abs().max()) <= 1e-5 * max(float(want.abs().max()), 1.0)
