@@ -106,6 +106,7 @@ static void rms_fw_into(const Tensor& x, const Tensor& gamma, int group, const T
 }
 static py::tuple rms_fw(const Tensor& x, const Tensor& gamma, int group, bool bf16) {
     Below guard;
+    if (group <= 0) refuse("rms_norm_forward: the group must be positive");
     Tensor y = fresh(x.sizes(), type_of(bf16), x), inv = fresh({x.size(0) * (x.size(1) / group)}, at::kFloat, x);
     rms_fw_into(x, gamma, group, y, inv, std::nullopt, 1e-6f);
     return py::make_tuple(y, inv);
@@ -271,7 +272,11 @@ static OptT linear_bw(const Tensor& dy_, const Tensor& x, const Tensor& w, const
 // One AdamW pass over (param, grad, m, v, decayed, bf16 shadow or None) tuples.
 static void adamw(const py::list& items, double wd, double lr, double b1, double b2, double eps, double bc1, double bc2, bool zero_grad) {
     std::vector<xlstm_adamw_desc> d(items.size());
-    auto at = [](const py::tuple& t, int i) -> const Tensor& { return THPVariable_Unpack(PyTuple_GET_ITEM(t.ptr(), i)); };
+    auto at = [](const py::tuple& t, int i) -> const Tensor& {
+        PyObject* o = PyTuple_GET_ITEM(t.ptr(), i);
+        if (!THPVariable_Check(o)) refuse("adamw: parameter, gradient and moments must be tensors");
+        return THPVariable_Unpack(o);
+    };
     for (size_t i = 0; i < d.size(); ++i) {
         const py::tuple t = items[i];
         const Tensor& p = at(t, 0);
