@@ -80,7 +80,10 @@ class MlstmShape:
         self.b, self.h, self.t, self.dqk, self.dhv, self.l = b, h, t, dqk, dhv, l
         self.dtype, self.gdtype, self.flags = dtype, gdtype, flags
         self.c = _lib.MlstmShape(b, h, t, dqk, dhv, l, _DT[dtype], _DT[gdtype], flags)
-        self.addr = ctypes.addressof(self.c)
+
+    @property
+    def addr(self):
+        return ctypes.addressof(self.c)
 
     def bh(self):
         return self.b * self.h
