@@ -523,8 +523,8 @@ struct Plan {
 static constexpr size_t kSmemCap = 220 * 1024;
 
 // Cycles of a step, the model the geometry is chosen by: every pass over NB sequences costs its FMAs (two warps a scheduler, R rows x NB sequences
-// x some columns a lane, two a packed FMA of two cycles) and some 900 cycles around them, and the last pass' exchange is exposed.
-static double step_cost(int R, int cols_per_lane, int NB, int nsub) { return nsub * (2.0 * cols_per_lane * R * NB + 900.0) + 900.0; }
+// x four columns a lane, two a packed FMA of two cycles) and some 900 cycles around them, and the last pass' exchange is exposed.
+static double step_cost(int R, int NB, int nsub) { return nsub * (8.0 * R * NB + 900.0) + 900.0; }
 
 // Batch groups: as many as there are SMs for, each with as few passes as that leaves.
 static bool groups_of(int B, int NB, int per_team, Args* a) {
@@ -552,7 +552,7 @@ static bool plan_fw(Args* out, Plan* best) {
             if (need > 32 || !groups_of(a.B, NB, a.NH * a.G, &a)) continue;
             p.smem = 4 * ((size_t)kWarps * 2 * p.R * NB + 2 * (size_t)KS * NB * 4 * a.UPC + 4 * (size_t)a.nsub * NB * a.UPC + 34 * (size_t)NB * a.UPC);
             p.words = 2 * (size_t)a.NH * a.B * a.dhd;
-            p.cost = step_cost(p.R, 4, NB, a.nsub);
+            p.cost = step_cost(p.R, NB, a.nsub);
             if (p.smem > kSmemCap || p.cost >= best->cost) continue;
             *out = a;
             *best = p;
@@ -577,11 +577,14 @@ static bool plan_bw(Args* out, Plan* best) {
             if (need > 32 || a.LPI < 1 || (senders + a.LPI - 1) / a.LPI > 2 * NB || !groups_of(a.B, NB, a.NH * a.G, &a)) continue;
             p.smem = 4 * (4 * (size_t)a.KH * p.R * NB + 20 * (size_t)NB * UPC + 2 * (size_t)a.nsub * NB * UPC + (p.R == 32 && NB == 8 ? 4 * 12 * kThr : 0));
             p.words = 2 * (size_t)a.NH * senders * a.B * a.dhd;
-            // many senders with all their words a step come in late enough that polling at once only gets in their way: 4 x 512 units, 8
-            // sequences 4.37 us a step without a rest, 4.34, 4.28, 3.95, 3.89, 3.96 after 150, 300, 450, 600, 800 cycles; fewer senders or
-            // words lose as much as they wait
-            a.rest = senders >= 24 && NB == 8 && a.nsub == 1 ? 600 : 0;
-            p.cost = step_cost(p.R, 4, NB, a.nsub);
+            // Many senders' words for eight sequences come in late enough that polling at once only gets in their way, where a thread has
+            // rows enough to multiply. us a step at 24 to 32 senders without a rest and after 600 cycles of it (sequences x heads x units):
+            //   32 rows  8 x 4 x 512 4.52 3.96   12 x 2 x 512 4.46 3.95   5 x 4 x 384 3.85 3.61   8 x 4 x 448 4.45 4.44   16 x 2 x 384 4.21 4.23
+            //   16 rows  12 x 4 x 256 3.56 3.28  32 x 2 x 256 3.54 3.29   32 x 2 x 192 3.69 3.58
+            //    8 rows  32 x 4 x 128 2.62 2.87  12 x 8 x 128 2.62 2.85
+            // With two sequences a pass, several passes or fewer senders, the wait is lost (up to 0.3 us); with four it would have to be shorter.
+            a.rest = senders >= 24 && NB == 8 && p.R >= 16 && a.nsub == 1 ? 600 : 0;
+            p.cost = step_cost(p.R, NB, a.nsub);
             if (p.smem > kSmemCap || p.cost >= best->cost) continue;
             *out = a;
             *best = p;
