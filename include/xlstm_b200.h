@@ -81,7 +81,8 @@ typedef struct {
 
 /* Bytes of the opaque chunk-state record the forward can leave for the backward
  * (the reference's cst/nst arrays, src/gpu/ops.rs:3955-3967). Passing saved=NULL to
- * both calls makes the backward recompute the chunk-boundary states instead. */
+ * both calls makes the backward recompute the chunk-boundary states instead. Its size and layout follow from
+ * B, H, T, dqk, dhv, L, dtype and flags; a backward may differ from its forward in gdtype alone. */
 size_t xlstm_mlstm_saved_bytes(const xlstm_mlstm_shape* s);
 size_t xlstm_mlstm_fw_workspace_bytes(const xlstm_mlstm_shape* s);
 size_t xlstm_mlstm_bw_workspace_bytes(const xlstm_mlstm_shape* s, int have_saved);

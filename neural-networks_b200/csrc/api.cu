@@ -50,14 +50,16 @@ static inline bool use_tc(const xlstm_mlstm_shape* s) {
 
 // The chunk-parallel kernels: square heads of 128 or 256 where eight launches instead of two pay. Measured, forward + backward in us:
 // at 256 they win as soon as the sequential kernels need two chunks (64 heads x 128: 145 -> 77; 256 x 256: 744 -> 359; 256 x 2048:
-// 5019 -> 2121). At 128 the one-CTA-per-head kernels cost 24 + 0.212 T per wave of heads however many heads there are, these some 70 + 0.0014 T
-// per head, or 0.00155 T with fp32 gradients: 4 x 512 118 -> 66, 64 x 1024 237 -> 165, 128 x 512 131 -> 156, 160 x 512 248 -> 198.
+// 5019 -> 2121). At 128 the one-CTA-per-head kernels cost 24 + 0.212 T per wave of heads however many heads there are, these some 70 + 0.00155 T
+// per head: 4 x 512 125 -> 77, 64 x 1024 241 -> 181, 128 x 512 140 -> 173, 160 x 512 252 -> 216. That is with fp32 gradients; with bf16 ones a
+// head costs 0.0014 T, and from 112 to 128 heads of 1024 to 2048 (and twice as many) up to 7 percent are left lying (128 x 2048: 471 against
+// 440). But the rule decides the layout of the state record, which a forward and a backward share that may differ in their gradients' type.
 static inline bool use_par(const xlstm_mlstm_shape* s) {
     if (!use_tc(s) || s->dqk != s->dhv || s->T > 128 * 2048) return false;
     if (s->dqk == 256) return s->T > 64;
     if (s->dqk != 128 || s->T <= 384) return false;
     const double bh = (double)s->B * s->H, waves = (double)((s->B * s->H + sm_count() - 1) / sm_count());
-    return 70 + (s->gdtype == XLSTM_F32 ? 0.00155 : 0.0014) * bh * s->T < 24 + 0.212 * s->T * waves;
+    return 70 + 0.00155 * bh * s->T < 24 + 0.212 * s->T * waves;
 }
 
 // Chunk-state record of the CUDA-core path: C then n, each the state ENTERING a chunk, f32.

@@ -77,3 +77,15 @@ def test_dp_entry_points_refuse_use_before_init():
     assert lib.xlstm_dp_bucket_start(0, None) < 0
     assert lib.xlstm_dp_wait(None) < 0
     assert lib.xlstm_dp_shutdown() == 0
+
+
+def test_the_state_record_does_not_depend_on_the_gradients_type():
+    """A backward may differ from its forward in the gradients' type alone, so the record between them may not."""
+    import ctypes
+    xl = importlib.import_module("neural-networks_b200")
+    lib, L = xl._lib.lib, xl._lib
+    for d in (64, 128, 256, 384):
+        for bh in (1, 8, 64, 80, 112, 128, 148, 160, 192, 256, 300):
+            for T in (1, 64, 65, 200, 385, 400, 512, 1024, 2048, 4096):
+                a, b = (L.MlstmShape(bh, 1, T, d, d, 64, L.BF16, g, 0) for g in (L.F32, L.BF16))
+                assert lib.xlstm_mlstm_saved_bytes(ctypes.byref(a)) == lib.xlstm_mlstm_saved_bytes(ctypes.byref(b)), (d, bh, T)

@@ -100,3 +100,19 @@ def test_states_that_start_at_any_float_are_read(shape):
         res.append((fused.ytil, *fused.state, *g[:5], *g[5]))
     assert xl._lib.lib.xlstm_device_status() == 0
     assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
+def test_a_record_serves_a_backward_of_the_other_gradient_width():
+    """64 heads of 400 positions, where the two gradient widths would be worth different kernels: a forward called with one gradient
+    type leaves the record that a backward called with the other reads."""
+    from gpu_util import ops, dev, mlstm_inputs
+    B, H, T, d = 8, 8, 400, 128
+    q, k, v, ig, fg, dy = mlstm_inputs(B, H, T, d, d, seed=76, bf16=True)
+    bf = torch.bfloat16
+    args, dyb = (dev(q, bf), dev(k, bf), dev(v, bf), dev(ig), dev(fg)), dev(dy, bf)
+    wide, narrow = (ops.MlstmShape(B, H, T, d, d, 64, bf, t) for t in (torch.float32, bf))
+    for fw, bw, g in ((wide, narrow, dyb), (narrow, wide, dyb.float())):
+        got = ops.mlstm_fused_bw(ops.mlstm_fused_fw(*args, fw), *args, g, bw)
+        want = ops.mlstm_fused_bw(ops.mlstm_fused_fw(*args, bw), *args, g, bw)
+        for a, b in zip(got[:5] + got[5], want[:5] + want[5]):
+            assert torch.equal(a, b)
