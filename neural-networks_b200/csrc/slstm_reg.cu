@@ -592,6 +592,18 @@ static bool plan_bw(Args* out, Plan* best) {
     return best->cost < 1e30;
 }
 
+// Where the device has no memory left to give (a host whose own runtime holds all of it), the call goes to the kernels of slstm.cu, which up to
+// 256 units a head need none beyond their arguments.
+#define XL_ROOM(expr)                                 \
+    do {                                              \
+        cudaError_t room__ = (expr);                  \
+        if (room__ == cudaErrorMemoryAllocation) {    \
+            (void)cudaGetLastError();                 \
+            return XLSTM_DECLINED;                    \
+        }                                             \
+        XL_CUDA(room__);                              \
+    } while (0)
+
 // The exchange words come from a memory pool of the library's own, in stream order: launches on several streams or threads each have theirs,
 // and the pool gives back what it holds beyond 32 MiB whenever the device is synchronised.
 static int pool_of(int dev, cudaMemPool_t* out) {
@@ -603,7 +615,7 @@ static int pool_of(int dev, cudaMemPool_t* out) {
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        XL_CUDA(cudaMemPoolCreate(&pools[dev], &props));
+        XL_ROOM(cudaMemPoolCreate(&pools[dev], &props));
         unsigned long long keep = 32ull << 20;
         XL_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
     }
@@ -616,7 +628,7 @@ static int start(cudaStream_t st, const void* kern, Args& a, const Plan& p, cons
     XL_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return XLSTM_DECLINED;
     const int grid = a.NH * a.teams * a.G;
-    XL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
+    XL_ROOM(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));  // loads the kernel on its first call
     int* status = tc_status_ptr();
     if (!status) return XLSTM_ERR_CUDA;
     if (getenv("XLSTM_DEBUG"))
@@ -627,7 +639,7 @@ static int start(cudaStream_t st, const void* kern, Args& a, const Plan& p, cons
     if (rc) return rc;
     void* mem = nullptr;
     const size_t bytes = 256 + p.words * sizeof(uint2);
-    XL_CUDA(cudaMallocFromPoolAsync(&mem, bytes, pool, st));
+    XL_ROOM(cudaMallocFromPoolAsync(&mem, bytes, pool, st));
     a.abort = (unsigned*)mem;
     a.ll = (uint2*)((char*)mem + 256);
     void* args[2] = {&a, &status};
