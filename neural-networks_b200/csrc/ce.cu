@@ -195,8 +195,8 @@ __device__ __forceinline__ float narrow_row(const float* z, float* d, bool live,
     const float k1 = 2.f * icap * 1.4426950408889634f, k2 = (CAP ? cap : 1.f) * 1.4426950408889634f;
     auto squash = [&](float x) { return CAP ? 1.f - __fdividef(2.f, 1.f + ex2(x * k1)) : x; };
     float v[VPL], e[VPL], mx = -INFINITY, sum = 0.f;
-    const bool any = tg < (uint32_t)C;  // a target that is no symbol: nothing is read or written for it, its probability is 0
-    const float zt = any ? squash(z[tg]) : 0.f;
+    const bool any = tg < (uint32_t)C;  // a target that is no symbol: its probability is 0, nothing is patched
+    const float zt = squash(z[any ? tg : 0u]);
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
         const int j = i * 32 + lane;
