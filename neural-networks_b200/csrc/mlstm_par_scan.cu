@@ -13,6 +13,9 @@ namespace par {
 // ---- gate vectors: one CTA per head, a warp per chunk, four consecutive positions per lane --------------------------------------
 // fc = cumulative log sigmoid(f) inside the chunk; m_t = fc_t + max(m_prev, max_{j<=t}(i_j - fc_j)); the chain of m_prev over the
 // chunks is NC dependent steps of one thread. FROM_M: m is given (backward), nothing is chained.
+// fc, i - fc and the chain are doubles: fc grows to tens over a chunk, and its rounding at 32 bits, added up along the chain, made m and the
+// weights of n (both fp32 results) two to four times less exact than the kernels with chunks of 64 positions (8 heads, 4069 positions: m 1.0e-7
+// there and 3.6e-7 here, now 0.4e-7; n 1.8e-7, 7.0e-7, 0.9e-7). Pairs of floats are as exact and take longer, in the chain above all.
 struct GateArgs {
     const float *ig, *fg, *m_in;
     float *m, *m_last;
@@ -20,10 +23,10 @@ struct GateArgs {
     int B, H, T, NC;
 };
 static constexpr int kMaxChunks = 2048;
-struct Local { float fc[4], um[4], u[4]; };
+struct Local { double fc[4], um[4], u[4]; };
 __device__ __forceinline__ Local chunk_local(const GateArgs& p, int b, int h, int ck, int lane) {
     Local r;
-    float s = 0.f, mx = -INFINITY;
+    double s = 0., mx = -INFINITY;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const int t = ck * LC + lane * 4 + e;
@@ -33,50 +36,52 @@ __device__ __forceinline__ Local chunk_local(const GateArgs& p, int b, int h, in
             f = p.fg[gi];
             i = p.ig[gi];
         }
-        s += log_sigmoid(f);
+        s += (double)log_sigmoid(f);
         r.fc[e] = s;
         r.u[e] = i;
     }
-    float pre = s;
+    double pre = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float y = __shfl_up_sync(0xffffffffu, pre, o);
+        const double y = __shfl_up_sync(0xffffffffu, pre, o);
         if (lane >= o) pre += y;
     }
-    const float before = __shfl_up_sync(0xffffffffu, pre, 1);
+    const double before = __shfl_up_sync(0xffffffffu, pre, 1);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         if (lane) r.fc[e] += before;
         r.u[e] -= r.fc[e];
-        mx = fmaxf(mx, r.u[e]);
+        mx = fmax(mx, r.u[e]);
         r.um[e] = mx;
     }
-    float pm = mx;
+    double pm = mx;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float y = __shfl_up_sync(0xffffffffu, pm, o);
-        if (lane >= o) pm = fmaxf(pm, y);
+        const double y = __shfl_up_sync(0xffffffffu, pm, o);
+        if (lane >= o) pm = fmax(pm, y);
     }
-    const float mb = __shfl_up_sync(0xffffffffu, pm, 1);
+    const double mb = __shfl_up_sync(0xffffffffu, pm, 1);
     if (lane)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r.um[e] = fmaxf(r.um[e], mb);
+        for (int e = 0; e < 4; ++e) r.um[e] = fmax(r.um[e], mb);
     return r;
 }
 template <bool FROM_M>
 __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
-    __shared__ float s_fc[FROM_M ? 1 : kMaxChunks], s_um[FROM_M ? 1 : kMaxChunks];
+    __shared__ double s_fc[FROM_M ? 1 : kMaxChunks], s_um[FROM_M ? 1 : kMaxChunks];
     const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H, w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const bool again = FROM_M || p.NC > nw;  // else a warp has one chunk, and keeps it
+    Local l;
     if (!FROM_M) {
         for (int ck = w; ck < p.NC; ck += nw) {
-            const Local l = chunk_local(p, b, h, ck, lane);
+            l = chunk_local(p, b, h, ck, lane);
             if (lane == 31) { s_fc[ck] = l.fc[3]; s_um[ck] = l.um[3]; }
         }
         __syncthreads();
         if (threadIdx.x == 0) {  // s_um becomes the m each chunk enters with
-            float m = p.m_in ? p.m_in[bh] : 0.f;
+            double m = p.m_in ? p.m_in[bh] : 0.f;
             for (int ck = 0; ck < p.NC; ++ck) {
-                const float next = s_fc[ck] + fmaxf(m, s_um[ck]);
+                const double next = s_fc[ck] + fmax(m, s_um[ck]);
                 s_um[ck] = m;
                 m = next;
             }
@@ -84,21 +89,22 @@ __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
         __syncthreads();
     }
     for (int ck = w; ck < p.NC; ck += nw) {
-        const Local l = chunk_local(p, b, h, ck, lane);
+        if (again) l = chunk_local(p, b, h, ck, lane);
         const int t0 = ck * LC;
-        float m_prev, m[4];
+        float m_in, m[4];  // as they are stored: what the entering state is scaled by, and what the backward will read
         if (FROM_M) {
-            m_prev = ck ? p.m[(size_t)bh * p.T + t0 - 1] : p.m_in ? p.m_in[bh] : 0.f;
+            m_in = ck ? p.m[(size_t)bh * p.T + t0 - 1] : p.m_in ? p.m_in[bh] : 0.f;
 #pragma unroll
             for (int e = 0; e < 4; ++e) m[e] = p.m[(size_t)bh * p.T + min(t0 + lane * 4 + e, p.T - 1)];
         } else {
-            m_prev = s_um[ck];
+            const double m_prev = s_um[ck];
+            m_in = (float)m_prev;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) m[e] = l.fc[e] + fmaxf(m_prev, l.um[e]);
+            for (int e = 0; e < 4; ++e) m[e] = (float)(l.fc[e] + fmax(m_prev, l.um[e]));
         }
         // m of the last position in the sequence (the scan's tree rounds the positions behind it differently)
         const int tl = min(p.T - 1 - t0, LC - 1);
-        const float fcL = __shfl_sync(0xffffffffu, l.fc[3], 31);
+        const double fcL = __shfl_sync(0xffffffffu, l.fc[3], 31);
         const float mL = __shfl_sync(0xffffffffu, (tl & 3) == 0 ? m[0] : (tl & 3) == 1 ? m[1] : (tl & 3) == 2 ? m[2] : m[3], tl >> 2);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -109,12 +115,13 @@ __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
                 p.m[(size_t)bh * p.T + t] = m[e];
                 if (t == p.T - 1 && p.m_last) p.m_last[bh] = m[e];
             }
-            p.v.rowt[o] = in ? l.fc[e] - m[e] : -INFINITY;  // past T the decay mask is 0 whatever colt is
-            p.v.colt[o] = l.u[e];
-            p.v.a[o] = in ? expf(fcL + l.u[e] - mL) : 0.f;
-            p.v.b[o] = in ? expf(l.fc[e] + m_prev - m[e]) : 0.f;
+            const double fm = l.fc[e] - m[e];
+            p.v.rowt[o] = in ? (float)fm : -INFINITY;  // past T the decay mask is 0 whatever colt is
+            p.v.colt[o] = (float)l.u[e];
+            p.v.a[o] = in ? expf((float)((fcL - mL) + l.u[e])) : 0.f;
+            p.v.b[o] = in ? expf((float)(fm + m_in)) : 0.f;
         }
-        if (lane == 0) p.v.g[(size_t)bh * p.NC + ck] = expf(fcL + m_prev - mL);
+        if (lane == 0) p.v.g[(size_t)bh * p.NC + ck] = expf((float)((fcL - mL) + m_in));
     }
 }
 int gates_launch(cudaStream_t st, const float* ig, const float* fg, const float* m_in, float* m, float* m_last, const Vecs& v,
@@ -288,6 +295,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
         constexpr int HC = NT / 2, PC = HC / 32;
         const uint32_t t0 = tC + ((uint32_t)(32 * qd) << 16) + half * HC;
         const size_t crow = ((size_t)bh * p.D + vi * 128 + row) * p.D + qi * NT + half * HC;
+        const bool c0_whole = p.c0 && ((uintptr_t)p.c0 & 15) == 0;
         for (int i = 0; i <= p.NC && !fail; ++i) {
             const bool last = i == p.NC;
             const int ck = last ? 0 : chunk(i);
@@ -303,7 +311,13 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
                 float v[32];
                 if (i == 0) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = p.c0 ? p.c0[crow + c * 32 + j] : 0.f;  // once a call; a caller's state may start at any float
+                    for (int j = 0; j < 32; j += 4) {  // a caller's state may start at any float
+                        const float* src = p.c0 + crow + c * 32 + j;
+                        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (c0_whole) x = *reinterpret_cast<const float4*>(src);
+                        else if (p.c0) x = make_float4(src[0], src[1], src[2], src[3]);
+                        v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
+                    }
                 } else {
                     tmem_ld32(t0 + c * 32, v);
                     tmem_ld_wait();

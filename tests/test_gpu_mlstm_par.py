@@ -116,3 +116,14 @@ def test_a_record_serves_a_backward_of_the_other_gradient_width():
         want = ops.mlstm_fused_bw(ops.mlstm_fused_fw(*args, bw), *args, g, bw)
         for a, b in zip(got[:5] + got[5], want[:5] + want[5]):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shape,carried", [((1, 4, 1500, 128), True), ((1, 2, 3000, 256), False), ((2, 2, 385, 128), True)])
+def test_stabiliser_and_normaliser_keep_their_fp32_precision(shape, carried):
+    """m and n are fp32 results that no product of the tensor cores enters. Each is rounded once where it is stored (6e-8) and inherits the
+    fp32 logarithms, exponentials and sums behind it, a few roundings more: 2e-7 for m, 4e-7 for n, whatever the number of chunks."""
+    got, ref, fused, _ = _run(shape, torch.float32, 77, carried, True)
+    B, H, T, _ = shape
+    for name, tol in (("m", 2e-7), ("mlast", 2e-7), ("n", 4e-7)):
+        a, b = got[name].reshape(-1), np.asarray(ref[name]).reshape(-1)
+        assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b), (name, np.linalg.norm(a - b) / np.linalg.norm(b))
