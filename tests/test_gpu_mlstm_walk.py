@@ -32,3 +32,23 @@ def test_walk_and_chunks_match_the_oracle(B, H, T, dqk, dhv, L, carried, save):
     ref.update(O.mlstm_core_bw(q, k, v, ig, fg, dy, B, H, T, dqk, dhv, **c0, **d0))
     for n, x in got.items():
         assert rel_to_max(host(x), ref[n]) <= 1e-4, n
+
+
+@pytest.mark.parametrize("T,carried", [(64, False), (300, False), (129, True)])
+def test_forget_gates_around_zero_do_not_cost_the_stabiliser_its_digits(T, carried):
+    """log sigmoid(0) = -0.69 a position: the gates' sum reaches -44 over a chunk, one unit in whose last place is 3.8e-6, while m stays a
+    number around 1. m_t is i_s plus the log gates of the few positions since s, each good to half a unit (3e-8) of its own, and is
+    rounded once itself (6e-8 at 1): within 3e-7."""
+    import torch
+    from gpu_util import ops, dev, host
+    B, H, d = 2, 3, 32
+    r = np.random.default_rng(T)
+    f32 = lambda a: a.astype(np.float32).astype(np.float64)
+    q, k, v = (f32(r.standard_normal((B * T, H * d))) for _ in range(3))
+    ig, fg = f32(0.5 * r.standard_normal((B * T, H))), f32(0.1 * r.standard_normal((B * T, H)))
+    c0 = (f32(r.standard_normal((B * H, d, d))), f32(r.standard_normal((B * H, d))), f32(r.standard_normal(B * H))) if carried else None
+    st = ops.MlstmShape(B, H, T, d, d, 64, torch.float32, torch.float32)
+    fused = ops.mlstm_fused_fw(*(dev(a) for a in (q, k, v, ig, fg)), st, carry_in=None if c0 is None else tuple(dev(a) for a in c0))
+    ref = O.mlstm_core_fw(q, k, v, ig, fg, B, H, T, d, d, **(dict(C0=c0[0], n0=c0[1], m0=c0[2]) if carried else {}))
+    assert np.abs(host(fused.msv) - ref["m"]).max() <= 3e-7
+    assert np.abs(host(fused.state[2]) - ref["mlast"]).max() <= 3e-7
