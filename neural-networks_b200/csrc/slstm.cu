@@ -1261,6 +1261,31 @@ static int run(cudaStream_t st, bool bwd, SlstmArgs a) {
 
 using namespace xl;
 
+// Sequences [b0, b0 + nb) of a call.
+template <typename A>
+static A slice(A a, int b0, int nb) {
+    const size_t state = (size_t)b0 * a.H, rows = state * a.T;
+    auto on = [](auto*& p, size_t n) { if (p) p += n; };
+    on(a.g, 4 * rows); on(a.dy, rows); on(a.out, rows);
+    on(a.c, state); on(a.n, state); on(a.m, state); on(a.h, state); on(a.dh, state); on(a.dc, state); on(a.dn, state);
+    on(a.s.c_prev, rows); on(a.s.n_prev, rows); on(a.s.ipr, rows); on(a.s.fpr, rows); on(a.s.c, rows); on(a.s.n, rows); on(a.s.zt, rows);
+    on(a.s.ot, rows); on(a.s.h_prev, rows);
+    a.B = nb;
+    return a;
+}
+// The register-resident kernels where they take the call, as many sequences at a time as they do; else the ones here.
+static int slices(cudaStream_t st, bool bwd, const SlstmArgs& a, const sreg::Args& r) {
+    const int per = slstm_reg_batch(r, bwd);
+    if (!per) return run(st, bwd, a);
+    for (int b0 = 0; b0 < a.B; b0 += per) {
+        const int nb = a.B - b0 < per ? a.B - b0 : per;
+        int rc = bwd ? slstm_reg_bw(st, slice(r, b0, nb)) : slstm_reg_fw(st, slice(r, b0, nb));
+        if (rc == XLSTM_DECLINED) rc = run(st, bwd, slice(a, b0, nb));
+        if (rc) return rc == XLSTM_DECLINED && b0 ? XLSTM_ERR_CUDA : rc;
+    }
+    return XLSTM_OK;
+}
+
 static int check_common(const char* who, const float* wh, const float* g, const xlstm_slstm_slabs* s, int B, int H,
                         int NH, int T) {
     XL_CHECK_ARG(wh && g && s, "%s: null pointer", who);
@@ -1283,9 +1308,7 @@ extern "C" int xlstm_slstm_fw(void* stream, const float* wh, float* g, const flo
     sreg::Args r = {};
     r.wh = wh; r.g = g; r.bcat = bcat; r.c = c; r.n = n; r.m = m; r.h = h; r.out = out; r.s = *slabs;
     r.B = B; r.H = H; r.NH = NH; r.T = T; r.carry = carry; r.dhd = H / NH;
-    rc = slstm_reg_fw((cudaStream_t)stream, r);
-    if (rc != XLSTM_DECLINED) return rc;
-    return run((cudaStream_t)stream, false, a);
+    return slices((cudaStream_t)stream, false, a, r);
 }
 
 extern "C" int xlstm_slstm_bw(void* stream, const float* wh, const float* dy, float* g, float* dh, float* dc,
@@ -1301,7 +1324,5 @@ extern "C" int xlstm_slstm_bw(void* stream, const float* wh, const float* dy, fl
     sreg::Args r = {};
     r.wh = wh; r.g = g; r.dy = dy; r.dh = dh; r.dc = dc; r.dn = dn; r.s = *slabs;
     r.B = B; r.H = H; r.NH = NH; r.T = T; r.carry = carry; r.dhd = H / NH;
-    rc = slstm_reg_bw((cudaStream_t)stream, r);
-    if (rc != XLSTM_DECLINED) return rc;
-    return run((cudaStream_t)stream, true, a);
+    return slices((cudaStream_t)stream, true, a, r);
 }

@@ -605,7 +605,8 @@ static bool plan_bw(Args* out, Plan* best) {
     } while (0)
 
 // The exchange words come from a memory pool of the library's own, in stream order: launches on several streams or threads each have theirs,
-// and the pool gives back what it holds beyond 32 MiB whenever the device is synchronised.
+// and the pool gives back what it holds beyond kPoolKeep whenever the device is synchronised.
+static constexpr size_t kPoolKeep = 32 << 20;
 static int pool_of(int dev, cudaMemPool_t* out) {
     static std::mutex mu;
     static cudaMemPool_t pools[64];
@@ -616,7 +617,7 @@ static int pool_of(int dev, cudaMemPool_t* out) {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         XL_ROOM(cudaMemPoolCreate(&pools[dev], &props));
-        unsigned long long keep = 32ull << 20;
+        unsigned long long keep = kPoolKeep;
         XL_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
     }
     *out = pools[dev];
@@ -669,6 +670,36 @@ static const void* bw_kernel(int R) {
 // The forward also needs two steps: the second one's exchange is what tells a CTA that the others have read the carried h it will overwrite.
 static bool takes(const Args& a) { return a.dhd % 16 == 0 && a.dhd <= 512 && a.T >= (a.dhd >= 256 ? 8 : 14) && a.T < (1 << 30); }
 
+// Large batches: a step takes a pass after the other over as many sequences as fit the SMs, while the cluster kernels take all that are resident
+// at once, and past that whole waves. Measured against them, 64 steps, us forward | backward (sequences x heads x units):
+//   one pass    32 x 4 x 256 335 -> 215 | 417 -> 262   64 x 2 x 160 246 -> 215 | 288 -> 270   128 x 4 x 64 195 -> 128 | 185 -> 187
+//               192 x 4 x 32 178 -> 119 | 140 -> 164   64 x 4 x 96  205 -> 170 | 198 -> 249 (backwards only the 32-unit CTAs of narrow heads lose)
+//   several     64 x 4 x 256 858 -> 404 | 991 -> 487   512 x 4 x 256 5033 -> 3076 | 5876 -> 4789   64 x 4 x 224 766 -> 415 | 900 -> 490
+//               64 x 4 x 512 2041 -> 1396 | 2584 -> 2024   128 x 4 x 240 1370 -> 1071 | 20 x 4 x 240 324 -> 384, 256 x 4 x 240 2832 -> 2963
+//               128 x 4 x 128 341 -> 316 | 402 -> 418  128 x 8 x 64 287 -> 240 | 243 -> 346   64 x 4 x 192 318 -> 403 | 382 -> 532
+//               64 x 4 x 160 285 -> 397 | 324 -> 567   256 x 4 x 48 224 -> 280 | 185 -> 379 (rows padded to a power of two)
+static bool pays(const Args& a, const Plan& p, bool bwd) {
+    const int d = a.dhd;
+    if (a.nsub == 1) return !bwd || d >= 128 || a.UPC < 32 || p.NB < 8;
+    return d > 256 || (d > 192 && (!bwd || d % 32 == 0)) || (!bwd && (d & (d - 1)) == 0);
+}
+
+// Sequences per launch: all, or as few equal slices as keep each one's words in what the pool holds on to (a larger allocation is mapped
+// anew, some 0.5 to 3 ms, after every synchronisation).
+static int batch_of(const Args& a, bool bwd) {
+    Args s = a;
+    for (int n = 1; n <= a.B; ++n) {
+        Plan p;
+        const int B = (a.B + n - 1) / n;
+        if (n > 1 && B == s.B) continue;
+        s = a;
+        s.B = B;
+        if (!(bwd ? plan_bw(&s, &p) : plan_fw(&s, &p)) || (n == 1 && !pays(s, p, bwd))) return 0;
+        if (256 + p.words * sizeof(uint2) <= kPoolKeep) return B;
+    }
+    return 0;
+}
+
 }  // namespace sreg
 
 static bool aligned(std::initializer_list<const void*> ptrs) {  // read and written 16 bytes at a time
@@ -677,18 +708,21 @@ static bool aligned(std::initializer_list<const void*> ptrs) {  // read and writ
     return true;
 }
 
+int slstm_reg_batch(const sreg::Args& a, bool bwd) {
+    const bool ok = bwd ? aligned({a.wh, a.dy, a.g, a.s.ot, a.s.c, a.s.n, a.s.fpr, a.s.ipr, a.s.zt, a.s.c_prev, a.s.n_prev})
+                        : aligned({a.g, a.out, a.s.c, a.s.n, a.s.fpr, a.s.ipr, a.s.zt, a.s.ot, a.s.c_prev, a.s.n_prev, a.s.h_prev});
+    return ok && sreg::takes(a) ? sreg::batch_of(a, bwd) : 0;
+}
+
 int slstm_reg_fw(cudaStream_t st, sreg::Args a) {
     sreg::Plan p;
-    if (!aligned({a.g, a.out, a.s.c, a.s.n, a.s.fpr, a.s.ipr, a.s.zt, a.s.ot, a.s.c_prev, a.s.n_prev, a.s.h_prev}) || !sreg::takes(a) ||
-        !sreg::plan_fw(&a, &p))
-        return XLSTM_DECLINED;
+    if (!sreg::plan_fw(&a, &p)) return XLSTM_DECLINED;
     return sreg::start(st, p.CG == 2 ? sreg::fw_kernel<2>(p) : sreg::fw_kernel<1>(p), a, p, "fw");
 }
 
 int slstm_reg_bw(cudaStream_t st, sreg::Args a) {
     sreg::Plan p;
-    if (!aligned({a.wh, a.dy, a.g, a.s.ot, a.s.c, a.s.n, a.s.fpr, a.s.ipr, a.s.zt, a.s.c_prev, a.s.n_prev}) || !sreg::takes(a) || !sreg::plan_bw(&a, &p))
-        return XLSTM_DECLINED;
+    if (!sreg::plan_bw(&a, &p)) return XLSTM_DECLINED;
     return sreg::start(st, p.NB == 8 ? sreg::bw_kernel<8>(p.R) : p.NB == 4 ? sreg::bw_kernel<4>(p.R) : sreg::bw_kernel<2>(p.R), a, p, "bw");
 }
 

@@ -104,7 +104,9 @@ __device__ __forceinline__ bool gather(float (&v)[M][N], const uint2* p, size_t 
 
 }  // namespace sreg
 
-// Whether the shape and the device take these kernels; launches them (XLSTM_DECLINED: not this shape).
+// Sequences that these kernels take in a launch (0: they do not take the call), and a launch over that many or fewer of them.
+// XLSTM_DECLINED: the device has no memory for the exchange words; nothing was launched.
+int slstm_reg_batch(const sreg::Args& a, bool bwd);
 int slstm_reg_fw(cudaStream_t st, sreg::Args a);
 int slstm_reg_bw(cudaStream_t st, sreg::Args a);
 
