@@ -101,7 +101,10 @@ int xlstm_mlstm_fw(void* stream, const xlstm_mlstm_shape* s, const void* q, cons
 
 /* The state a call would end in, without its outputs: the recurrence over (C, n, m) alone, about half a
  * forward's time. New (the reference has no such entry): context parallelism summarises a segment with it
- * before the carry from the ranks to its left is known. Arguments as in xlstm_mlstm_fw; out_* required. */
+ * before the carry from the ranks to its left is known. Arguments as in xlstm_mlstm_fw; out_* required. The
+ * bits are the forward's where that runs on the kernels of one CTA per head; where it runs on the
+ * chunk-parallel ones (square heads of 256 beyond 64 positions, of 128 beyond 384 where there are few enough),
+ * whose chunks are twice as long, the two agree to rounding. */
 int xlstm_mlstm_final_state(void* stream, const xlstm_mlstm_shape* s, const void* q, const void* k,
                             const void* v, const float* ig, const float* fg, const float* carry_C,
                             const float* carry_n, const float* carry_m, float* out_C, float* out_n,

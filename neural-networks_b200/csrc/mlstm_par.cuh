@@ -49,7 +49,7 @@ struct ScanArgs {           // one state recurrence: forward over (a.V, K) or ba
     const float* w;         // [BH][Tp]: weights of n's sum; forward: also scales x
     const float* g;         // [BH][NC]
     const float *c0, *n0;   // state the walk starts from, fp32 [BH][D][D], [BH][D], or null = 0
-    void* recC;             // bf16 [BH][entries][D][D] or null; entry k: the state before chunk k's update
+    void* recC;             // bf16 [BH][entries][D][D]; entry k: the state before chunk k's update
     float* recn;
     float *oC, *on;         // state after the walk, or null
     int B, H, T, D, NC, entries;

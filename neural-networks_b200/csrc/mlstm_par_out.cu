@@ -270,11 +270,9 @@ size_t mlstm_par_fw_workspace_bytes(int B, int H, int T, int d) {  // the record
     return vecs_bytes(B * H, (T + LC - 1) / LC, false) + mlstm_par_saved_bytes(B, H, T, d);
 }
 
-// states_only: the record (when `saved`) and the final state alone; `a.msv` may then be null.
 int mlstm_par_fw_launch(cudaStream_t st, const MlstmFwArgs& a, void* saved, void* workspace, size_t workspace_bytes) {
     const int NC = (a.T + LC - 1) / LC, BH = a.B * a.H, d = a.dqk;
-    const size_t vb = vecs_bytes(BH, NC, false), mb = a.msv ? 0 : align_up((size_t)BH * a.T * 4, 256);
-    const size_t need = vb + mb + (saved || a.states_only ? 0 : mlstm_par_saved_bytes(a.B, a.H, a.T, d));
+    const size_t vb = vecs_bytes(BH, NC, false), need = vb + (saved ? 0 : mlstm_par_saved_bytes(a.B, a.H, a.T, d));
     if (!workspace || workspace_bytes < need) {
         set_error("mlstm_fw: workspace of %zu B is smaller than the %zu B required", workspace_bytes, need);
         return XLSTM_ERR_WORKSPACE;
@@ -285,16 +283,15 @@ int mlstm_par_fw_launch(cudaStream_t st, const MlstmFwArgs& a, void* saved, void
     }
     char* ws = (char*)workspace;
     const Vecs v = vecs_at(ws, BH, NC, false);
-    float* m = a.msv ? a.msv : (float*)(ws + vb);
-    if (!saved && !a.states_only) saved = ws + vb + mb;
-    int rc = gates_launch(st, a.ig, a.fg, a.cm, m, a.om, v, a.B, a.H, a.T, NC, false);
+    if (!saved) saved = ws + vb;
+    int rc = gates_launch(st, a.ig, a.fg, a.cm, a.msv, a.om, v, a.B, a.H, a.T, NC, false);
     if (rc) return rc;
     ScanArgs s = {};
     s.x = a.v; s.y = a.k; s.w = v.a; s.g = v.g; s.c0 = a.cC; s.n0 = a.cn;
-    s.recC = saved; s.recn = saved ? (float*)((char*)saved + record_C_bytes(BH, NC, d)) : nullptr;
+    s.recC = saved; s.recn = (float*)((char*)saved + record_C_bytes(BH, NC, d));
     s.oC = a.oC; s.on = a.on; s.B = a.B; s.H = a.H; s.T = a.T; s.D = d; s.NC = NC; s.entries = NC + 1; s.bwd = false;
     rc = scan_launch(st, s);
-    if (rc || a.states_only) return rc;
+    if (rc) return rc;
     OutP p = {};
     if (!tc_make_map4(&p.tq, a.q, 2, a.B, a.T, a.H * d, 128, 2) || !tc_make_map4(&p.tk, a.k, 2, a.B, a.T, a.H * d, 128, 2) ||
         !tc_make_map4(&p.tv, a.v, 2, a.B, a.T, a.H * d, 128, 2) || !tc_make_map4(&p.ty, a.ytil, 2, a.B, a.T, a.H * d, 128, 2) ||
@@ -302,7 +299,7 @@ int mlstm_par_fw_launch(cudaStream_t st, const MlstmFwArgs& a, void* saved, void
         set_error("mlstm_fw: cuTensorMapEncodeTiled failed");
         return XLSTM_ERR_CUDA;
     }
-    p.v = v; p.recn = s.recn; p.m = m; p.psiv = a.psiv; p.qnv = a.qnv; p.H = a.H; p.T = a.T; p.NC = NC; p.units = BH * NC * (d / 128);
+    p.v = v; p.recn = s.recn; p.m = a.msv; p.psiv = a.psiv; p.qnv = a.qnv; p.H = a.H; p.T = a.T; p.NC = NC; p.units = BH * NC * (d / 128);
     p.status = tc_status_ptr();
     if (!p.status) return XLSTM_ERR_CUDA;
     return d == 128 ? out_run<1>(st, p) : out_run<2>(st, p);

@@ -143,7 +143,7 @@ struct ScanP {
     CUtensorMap tx, ty, trec;
     const float *w, *g, *c0, *n0;
     float *recn, *oC, *on;
-    int H, T, D, NC, Tp, entries, nv, nt, record;
+    int H, T, D, NC, Tp, entries, nv, nt;
     int* status;
 };
 static constexpr int kStateThreads = 256, kAuxThreads = 256;
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
                 fail = named_barrier_or(2, kAuxThreads, fail);
                 if (fail) break;
                 if (at < NT) {
-                    if (p.recn) p.recn[((size_t)bh * p.entries + ck) * p.D + qi * NT + at] = nn;
+                    p.recn[((size_t)bh * p.entries + ck) * p.D + qi * NT + at] = nn;
                     float s = 0.f;
 #pragma unroll
                     for (int r = 0; r < RG; ++r) s += red[r * NT + at];
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
             }
         }
         if (do_n && at < NT && !fail) {
-            if (!BWD && p.recn) p.recn[((size_t)bh * p.entries + p.NC) * p.D + qi * NT + at] = nn;
+            if (!BWD) p.recn[((size_t)bh * p.entries + p.NC) * p.D + qi * NT + at] = nn;
             if (p.on) p.on[(size_t)bh * p.D + qi * NT + at] = nn;
         }
     } else {
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
             if (i) PAR_WAIT(cdone, (i - 1) & 1);
             tc_fence_after();
             const float g = last ? 1.f : sg[ck];
-            const bool rec = p.record && (!last || !BWD);
+            const bool rec = !last || !BWD;
             if (rec && tid == 0) tma_store_wait_read();
             fail = named_barrier_or(1, kStateThreads, fail);  // the previous entry has left the staging buffer; all warps leave together
             if (fail) break;
@@ -391,7 +391,7 @@ int scan_launch(cudaStream_t st, const ScanArgs& a) {
     p.status = tc_status_ptr();
     if (!p.status) return XLSTM_ERR_CUDA;
     p.w = a.w; p.g = a.g; p.c0 = a.c0; p.n0 = a.n0; p.recn = a.recn; p.oC = a.oC; p.on = a.on;
-    p.H = a.H; p.T = a.T; p.D = a.D; p.NC = a.NC; p.Tp = a.NC * LC; p.entries = a.entries; p.record = a.recC != nullptr;
+    p.H = a.H; p.T = a.T; p.D = a.D; p.NC = a.NC; p.Tp = a.NC * LC; p.entries = a.entries;
     p.nv = a.D / 128;
     // columns per CTA: the narrowest block whose launch is still one wave (a narrow block's state pass and products are shorter, but
     // every block reads all of X), else the widest
@@ -399,7 +399,7 @@ int scan_launch(cudaStream_t st, const ScanArgs& a) {
     while (nt < a.D && a.B * a.H * p.nv * (a.D / nt) > sm_count()) nt *= 2;
     p.nt = a.D / nt;
     if (!tc_make_map4(&p.tx, a.x, 2, a.B, a.T, a.H * a.D, 64, 2) || !tc_make_map4(&p.ty, a.y, 2, a.B, a.T, a.H * a.D, 64, nt / 64) ||
-        (a.recC && !tc_make_map4(&p.trec, a.recC, 2, 1, (uint64_t)a.B * a.H * a.entries * a.D, a.D, 128, nt / 64))) {
+        !tc_make_map4(&p.trec, a.recC, 2, 1, (uint64_t)a.B * a.H * a.entries * a.D, a.D, 128, nt / 64)) {
         set_error("mlstm: cuTensorMapEncodeTiled failed");
         return XLSTM_ERR_CUDA;
     }

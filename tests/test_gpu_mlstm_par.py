@@ -127,3 +127,19 @@ def test_stabiliser_and_normaliser_keep_their_fp32_precision(shape, carried):
     for name, tol in (("m", 2e-7), ("mlast", 2e-7), ("n", 4e-7)):
         a, b = got[name].reshape(-1), np.asarray(ref[name]).reshape(-1)
         assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b), (name, np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 400, 128), (2, 1, 130, 256)])
+def test_final_state_alone_agrees_with_a_chunk_parallel_forward(shape):
+    """The states-only entry point keeps the kernels of one CTA per head: C within the bf16 products' bar, n and m to fp32 rounding."""
+    from gpu_util import ops, dev, host, mlstm_inputs, rel_to_max
+    B, H, T, d = shape
+    q, k, v, ig, fg, _ = mlstm_inputs(B, H, T, d, d, seed=78, bf16=True)
+    r = np.random.default_rng(79)
+    cin = tuple(dev(a) for a in (r.standard_normal((B * H, d, d)), r.standard_normal((B * H, d)), r.standard_normal((B * H,))))
+    bf = torch.bfloat16
+    st = ops.MlstmShape(B, H, T, d, d, 64, bf, torch.float32)
+    args = (dev(q, bf), dev(k, bf), dev(v, bf), dev(ig), dev(fg), st)
+    full, alone = ops.mlstm_fused_fw(*args, carry_in=cin).state, ops.mlstm_final_state(*args, carry_in=cin)
+    for a, b, tol in zip(alone, full, (2e-2, 2e-6, 2e-6)):
+        assert rel_to_max(host(a), host(b)) <= tol
