@@ -54,6 +54,10 @@ extern "C" {
  * for a state or a state gradient, or has T > 32 is refused. Ignored where the tensor-core path does not apply or the
  * heads are not 128 x 128 (the call then runs as without the flag). Results are those of the unpacked call. */
 #define XLSTM_PACK_SHORT 2u
+/* One span of a training sweep (a long sequence cut into calls that hand states on and gradients back): the chunk-parallel
+ * kernels then sum the gates in fp32, as in a call over the whole sequence, where a state that is a result of its own gets
+ * 64-bit sums. Set it on the forward call and on its backward call alike; ignored by the other kernels. */
+#define XLSTM_SWEEP 4u
 
 int xlstm_version(void);
 const char* xlstm_last_error(void);
@@ -132,11 +136,16 @@ int xlstm_mlstm_bw(void* stream, const xlstm_mlstm_shape* s, const void* q, cons
  *   state c,n,m,h [B,H]: read when carry!=0 (else zero), always written.
  *   slabs: nine [B,T,H] records in this order:
  *       c_prev, n_prev, i', f', c, n, z, o, h_prev   (src/gpu/ops.rs:2206-2256).
- * Heads of up to 256 units run on thread-block clusters. Wider heads (dense H up to 1024, block-diagonal
- * heads up to 512 units) run as ONE cooperative launch spanning the GPU, whose CTAs wait on one another
- * with bounded polls (a timeout shows in xlstm_device_status); that path uses barrier words, a 2 MiB
- * exchange array and (backward) a grow-only exchange buffer held by the library per device, so keep
- * those calls on one stream per device, as the reference keeps all its calls. Anything wider returns 1.
+ * Heads of a multiple of 16 and up to 512 units, from 8 steps on (14 below 256 units), run as cooperative
+ * launches whose CTAs wait on one another with bounded polls (a timeout shows in xlstm_device_status); their
+ * exchange words come from a stream-ordered memory pool of the library's own, which keeps at most 32 MiB
+ * between synchronisations, so launches on several streams are independent. Where that pool can get no
+ * memory, and for shorter calls, other widths and batches of narrow heads so large that they measure faster
+ * there, heads of up to 256 units run on thread-block clusters, which need nothing beyond the arguments.
+ * What is left (dense H up to 1024, short calls of wider heads) runs as ONE cooperative launch spanning the
+ * GPU that uses barrier words, a 2 MiB exchange array and (backward) a grow-only exchange buffer held by the
+ * library per device: keep those calls on one stream per device, as the reference keeps all its calls.
+ * Anything wider returns 1. Tensors that do not start on 16 bytes are taken, by the kernels that do not need it.
  */
 typedef struct {
     float *c_prev, *n_prev, *ipr, *fpr, *c, *n, *zt, *ot, *h_prev;

@@ -16,6 +16,7 @@ OK, DECLINED = 0, 1
 F32, BF16 = 0, 1
 FORCE_SIMT = 1
 PACK_SHORT = 2
+SWEEP = 4
 
 
 class MlstmShape(ctypes.Structure):

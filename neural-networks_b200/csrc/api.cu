@@ -178,6 +178,7 @@ extern "C" int xlstm_mlstm_fw(void* stream, const xlstm_mlstm_shape* s, const vo
     if (use_tc(s)) {
         const int npk = tc_pack_count(s, a.cC || a.oC);
         if (npk < 0) return XLSTM_ERR_ARG;
+        a.exact = !(s->flags & XLSTM_SWEEP);
         if (use_par(s)) return mlstm_par_fw_launch((cudaStream_t)stream, a, saved, workspace, workspace_bytes);
         return tc_fw_maybe_packed((cudaStream_t)stream, npk, a, saved, workspace, workspace_bytes);
     }
@@ -231,6 +232,7 @@ extern "C" int xlstm_mlstm_bw(void* stream, const xlstm_mlstm_shape* s, const vo
             a.qnv = qnv; a.dytil = d_ytil; a.cdC = carry_dC; a.cdn = carry_dn;
             a.dq = dq; a.dk = dk; a.dv = dv; a.dig = dig; a.dfg = dfg; a.odC = out_dC; a.odn = out_dn;
             a.B = s->B; a.H = s->H; a.T = s->T; a.dqk = s->dqk; a.dhv = s->dhv;
+            a.exact = !(s->flags & XLSTM_SWEEP);
             return mlstm_par_bw_launch(st, a, carry_C, carry_n, saved, s->gdtype, ws, ws_left);
         }
         if (!saved) {

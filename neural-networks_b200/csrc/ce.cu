@@ -332,7 +332,8 @@ static int ce_run(void* stream, const float* logits, const uint32_t* targets, co
     float* cta_loss = (float*)workspace;  // one sum per CTA, never more CTAs than rows
     int grid;
     if (C <= 1024 && !(((uintptr_t)logits | (uintptr_t)dlogits) & 15)) {
-        // tiles of about 24 KB, fewer rows where that leaves SMs without one; three CTAs of three stages fill an SM's shared memory
+        // tiles of at most 24 KB in whole groups of eight rows (257 columns: 16 rows, 16 KB), fewer rows where that leaves SMs without one;
+        // an SM's shared memory holds three CTAs of three such stages at 24 KB, four at 257 columns
         int RT = (24 * 1024 / (4 * C)) / 8 * 8;
         const int fair = (rows / sm_count() + 7) / 8 * 8;
         if (RT > fair) RT = fair;

@@ -13,6 +13,7 @@ struct MlstmFwArgs {
     float *savedC, *savedn;     // [BH, NC, dhv*dqk], [BH, NC, dqk]: state entering each chunk (may be null)
     float *oC, *on, *om;        // state after the last position (may be null)
     int B, H, T, dqk, dhv, L, NC;
+    int exact;                  // chunk-parallel path: 64-bit gate sums where the call takes or leaves a state
     int states_only;            // 1: walk the state recurrence only (recompute pass of the backward)
     int pass;                   // CUDA-core path, set by its launcher: 0 all in one walk, 1 the states (and msv), 2 a chunk's outputs
     // tensor-core path, packed mode (0 = off): T = npack * seg positions hold npack independent sequences of seg
@@ -33,6 +34,7 @@ struct MlstmBwArgs {
     float *dig, *dfg;
     float *odC, *odn;
     int B, H, T, dqk, dhv, L, NC;
+    int exact;                  // as in MlstmFwArgs
     int seg, npack;             // packed mode of the tensor-core path, as in MlstmFwArgs
     // CUDA-core path: record of dC, dn entering each chunk from its right ([BH, NC, dhv*dqk], [BH, NC, dqk]; null: one walk), and the pass
     float *recC, *recn;

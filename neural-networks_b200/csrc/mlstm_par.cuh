@@ -57,7 +57,7 @@ struct ScanArgs {           // one state recurrence: forward over (a.V, K) or ba
 };
 int scan_launch(cudaStream_t st, const ScanArgs& a);
 int gates_launch(cudaStream_t st, const float* ig, const float* fg, const float* m_in, float* m, float* m_last, const Vecs& v,
-                 int B, int H, int T, int NC, bool from_m);
+                 int B, int H, int T, int NC, bool from_m, bool exact);
 
 // Eight or four k16 steps of a product, issued by a converged warp. Descriptor arithmetic stays out of the loop: a step is a constant
 // added to the start address field (K-major: 32 bytes a step, four steps to a tile; MN-major: sixteen 128-byte rows a step).

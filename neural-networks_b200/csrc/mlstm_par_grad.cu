@@ -523,7 +523,7 @@ int mlstm_par_bw_launch(cudaStream_t st, const MlstmBwArgs& a, const float* carr
     float* pu = (float*)(ws + w.dc + w.dnn);
     float* pw = (float*)(ws + w.dc + w.dnn + w.dots);
     void* rec = ws + w.dc + w.dnn + 2 * w.dots;
-    int rc = gates_launch(st, a.ig, a.fg, a.cm, const_cast<float*>(a.msv), nullptr, v, a.B, a.H, a.T, NC, true);
+    int rc = gates_launch(st, a.ig, a.fg, a.cm, const_cast<float*>(a.msv), nullptr, v, a.B, a.H, a.T, NC, true, a.exact && a.cm);
     if (rc) return rc;
     ScanArgs s = {};
     s.g = v.g; s.B = a.B; s.H = a.H; s.T = a.T; s.D = d; s.NC = NC;

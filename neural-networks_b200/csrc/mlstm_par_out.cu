@@ -284,7 +284,7 @@ int mlstm_par_fw_launch(cudaStream_t st, const MlstmFwArgs& a, void* saved, void
     char* ws = (char*)workspace;
     const Vecs v = vecs_at(ws, BH, NC, false);
     if (!saved) saved = ws + vb;
-    int rc = gates_launch(st, a.ig, a.fg, a.cm, a.msv, a.om, v, a.B, a.H, a.T, NC, false);
+    int rc = gates_launch(st, a.ig, a.fg, a.cm, a.msv, a.om, v, a.B, a.H, a.T, NC, false, a.exact && (a.cm || a.om));
     if (rc) return rc;
     ScanArgs s = {};
     s.x = a.v; s.y = a.k; s.w = v.a; s.g = v.g; s.c0 = a.cC; s.n0 = a.cn;

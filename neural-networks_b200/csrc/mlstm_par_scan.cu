@@ -13,9 +13,11 @@ namespace par {
 // ---- gate vectors: one CTA per head, a warp per chunk, four consecutive positions per lane --------------------------------------
 // fc = cumulative log sigmoid(f) inside the chunk; m_t = fc_t + max(m_prev, max_{j<=t}(i_j - fc_j)); the chain of m_prev over the
 // chunks is NC dependent steps of one thread. FROM_M: m is given (backward), nothing is chained.
-// fc, i - fc and the chain are doubles: fc grows to tens over a chunk, and its rounding at 32 bits, added up along the chain, made m and the
-// weights of n (both fp32 results) two to four times less exact than the kernels with chunks of 64 positions (8 heads, 4069 positions: m 1.0e-7
-// there and 3.6e-7 here, now 0.4e-7; n 1.8e-7, 7.0e-7, 0.9e-7). Pairs of floats are as exact and take longer, in the chain above all.
+// A call that takes or leaves a state as a result (F = double) sums the gates and chains m in 64 bits: fc grows to tens over a chunk, and its rounding at
+// 32, added up along the chain, made m and n, then results of the call, two to four times less exact than the kernels with chunks of 64
+// positions (8 heads, 4069 positions: m 1.0e-7 there and 3.6e-7 here, now 0.4e-7; n 1.8e-7, 7.0e-7, 0.9e-7). Pairs of floats are as exact and
+// take longer, in the chain above all. Within a training step (no state, or XLSTM_SWEEP) m and n only weigh bf16 products, 1e-3 off themselves,
+// and floats do.
 struct GateArgs {
     const float *ig, *fg, *m_in;
     float *m, *m_last;
@@ -23,10 +25,14 @@ struct GateArgs {
     int B, H, T, NC;
 };
 static constexpr int kMaxChunks = 2048;
-struct Local { double fc[4], um[4], u[4]; };
-__device__ __forceinline__ Local chunk_local(const GateArgs& p, int b, int h, int ck, int lane) {
-    Local r;
-    double s = 0., mx = -INFINITY;
+__device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double larger(double a, double b) { return fmax(a, b); }
+template <typename F>
+struct Local { F fc[4], um[4], u[4]; };
+template <typename F>
+__device__ __forceinline__ Local<F> chunk_local(const GateArgs& p, int b, int h, int ck, int lane) {
+    Local<F> r;
+    F s = 0, mx = -INFINITY;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const int t = ck * LC + lane * 4 + e;
@@ -36,52 +42,52 @@ __device__ __forceinline__ Local chunk_local(const GateArgs& p, int b, int h, in
             f = p.fg[gi];
             i = p.ig[gi];
         }
-        s += (double)log_sigmoid(f);
+        s += (F)log_sigmoid(f);
         r.fc[e] = s;
         r.u[e] = i;
     }
-    double pre = s;
+    F pre = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffu, pre, o);
+        const F y = __shfl_up_sync(0xffffffffu, pre, o);
         if (lane >= o) pre += y;
     }
-    const double before = __shfl_up_sync(0xffffffffu, pre, 1);
+    const F before = __shfl_up_sync(0xffffffffu, pre, 1);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         if (lane) r.fc[e] += before;
         r.u[e] -= r.fc[e];
-        mx = fmax(mx, r.u[e]);
+        mx = larger(mx, r.u[e]);
         r.um[e] = mx;
     }
-    double pm = mx;
+    F pm = mx;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffu, pm, o);
-        if (lane >= o) pm = fmax(pm, y);
+        const F y = __shfl_up_sync(0xffffffffu, pm, o);
+        if (lane >= o) pm = larger(pm, y);
     }
-    const double mb = __shfl_up_sync(0xffffffffu, pm, 1);
+    const F mb = __shfl_up_sync(0xffffffffu, pm, 1);
     if (lane)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r.um[e] = fmax(r.um[e], mb);
+        for (int e = 0; e < 4; ++e) r.um[e] = larger(r.um[e], mb);
     return r;
 }
-template <bool FROM_M>
+template <bool FROM_M, typename F>
 __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
-    __shared__ double s_fc[FROM_M ? 1 : kMaxChunks], s_um[FROM_M ? 1 : kMaxChunks];
+    __shared__ F s_fc[FROM_M ? 1 : kMaxChunks], s_um[FROM_M ? 1 : kMaxChunks];
     const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H, w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const bool again = FROM_M || p.NC > nw;  // else a warp has one chunk, and keeps it
-    Local l;
+    Local<F> l;
     if (!FROM_M) {
         for (int ck = w; ck < p.NC; ck += nw) {
-            l = chunk_local(p, b, h, ck, lane);
+            l = chunk_local<F>(p, b, h, ck, lane);
             if (lane == 31) { s_fc[ck] = l.fc[3]; s_um[ck] = l.um[3]; }
         }
         __syncthreads();
         if (threadIdx.x == 0) {  // s_um becomes the m each chunk enters with
-            double m = p.m_in ? p.m_in[bh] : 0.f;
+            F m = p.m_in ? p.m_in[bh] : 0.f;
             for (int ck = 0; ck < p.NC; ++ck) {
-                const double next = s_fc[ck] + fmax(m, s_um[ck]);
+                const F next = s_fc[ck] + larger(m, s_um[ck]);
                 s_um[ck] = m;
                 m = next;
             }
@@ -89,7 +95,7 @@ __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
         __syncthreads();
     }
     for (int ck = w; ck < p.NC; ck += nw) {
-        if (again) l = chunk_local(p, b, h, ck, lane);
+        if (again) l = chunk_local<F>(p, b, h, ck, lane);
         const int t0 = ck * LC;
         float m_in, m[4];  // as they are stored: what the entering state is scaled by, and what the backward will read
         if (FROM_M) {
@@ -97,14 +103,14 @@ __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) m[e] = p.m[(size_t)bh * p.T + min(t0 + lane * 4 + e, p.T - 1)];
         } else {
-            const double m_prev = s_um[ck];
+            const F m_prev = s_um[ck];
             m_in = (float)m_prev;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) m[e] = (float)(l.fc[e] + fmax(m_prev, l.um[e]));
+            for (int e = 0; e < 4; ++e) m[e] = (float)(l.fc[e] + larger(m_prev, l.um[e]));
         }
         // m of the last position in the sequence (the scan's tree rounds the positions behind it differently)
         const int tl = min(p.T - 1 - t0, LC - 1);
-        const double fcL = __shfl_sync(0xffffffffu, l.fc[3], 31);
+        const F fcL = __shfl_sync(0xffffffffu, l.fc[3], 31);
         const float mL = __shfl_sync(0xffffffffu, (tl & 3) == 0 ? m[0] : (tl & 3) == 1 ? m[1] : (tl & 3) == 2 ? m[2] : m[3], tl >> 2);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -115,21 +121,22 @@ __global__ void __launch_bounds__(1024) par_gates(const GateArgs p) {
                 p.m[(size_t)bh * p.T + t] = m[e];
                 if (t == p.T - 1 && p.m_last) p.m_last[bh] = m[e];
             }
-            const double fm = l.fc[e] - m[e];
-            p.v.rowt[o] = in ? (float)fm : -INFINITY;  // past T the decay mask is 0 whatever colt is
+            p.v.rowt[o] = in ? (float)(l.fc[e] - m[e]) : -INFINITY;  // past T the decay mask is 0 whatever colt is
             p.v.colt[o] = (float)l.u[e];
-            p.v.a[o] = in ? expf((float)((fcL - mL) + l.u[e])) : 0.f;
-            p.v.b[o] = in ? expf((float)(fm + m_in)) : 0.f;
+            p.v.a[o] = in ? expf((float)(fcL + l.u[e] - mL)) : 0.f;
+            p.v.b[o] = in ? expf((float)(l.fc[e] + m_in - m[e])) : 0.f;
         }
-        if (lane == 0) p.v.g[(size_t)bh * p.NC + ck] = expf((float)((fcL - mL) + m_in));
+        if (lane == 0) p.v.g[(size_t)bh * p.NC + ck] = expf((float)(fcL + m_in - mL));
     }
 }
 int gates_launch(cudaStream_t st, const float* ig, const float* fg, const float* m_in, float* m, float* m_last, const Vecs& v,
-                 int B, int H, int T, int NC, bool from_m) {
+                 int B, int H, int T, int NC, bool from_m, bool exact) {
     GateArgs p = {ig, fg, m_in, m, m_last, v, B, H, T, NC};
     const int threads = NC >= 32 ? 1024 : 32 * NC;
-    if (from_m) par_gates<true><<<B * H, threads, 0, st>>>(p);
-    else par_gates<false><<<B * H, threads, 0, st>>>(p);
+    if (from_m && exact) par_gates<true, double><<<B * H, threads, 0, st>>>(p);
+    else if (from_m) par_gates<true, float><<<B * H, threads, 0, st>>>(p);
+    else if (exact) par_gates<false, double><<<B * H, threads, 0, st>>>(p);
+    else par_gates<false, float><<<B * H, threads, 0, st>>>(p);
     XL_LAUNCH_OK("par_gates");
     return XLSTM_OK;
 }
