@@ -254,6 +254,9 @@ int xlstm_colsum_narrow(void* stream, const void* x, int x_dtype, int rows, int 
 /* out[r][c] = bias[c] (+ residual[r][c] when given): the seed a projection's GEMM accumulates into with beta = 1
  * (broadcast_row / broadcast_row_resid, src/gpu/cuda/common.cu:20-48). f32, [rows, cols]. */
 int xlstm_bias_rows(void* stream, const float* residual, const float* bias, float* out, int rows, int cols);
+/* out_bf16[i] = bf16(scale[i] * x[i]) for up to eight vectors of n[i] floats in one launch: the biases that a cell's narrowed
+ * projections add in their epilogues. */
+int xlstm_narrow_vectors(void* stream, const float* const* x, void* const* out_bf16, const int* n, const float* scale, int count);
 
 /* Embedding backward without float atomics (replaces embedding_scatter_add / embedding_scatter_merge,
  * src/gpu/cuda/common.cu:127-168): table_g[id] += sum of the rows d[pos] with ids[pos] == id, in ascending

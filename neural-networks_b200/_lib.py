@@ -80,6 +80,7 @@ SIGNATURES = {
     "xlstm_colsum_workspace_bytes": (_sz, [_i, _i]),
     "xlstm_colsum_narrow": (_i, [_vp, _vp, _i, _i, _i, _f, _vp, _vp, _vp, _sz]),
     "xlstm_bias_rows": (_i, [_vp, _vp, _vp, _vp, _i, _i]),
+    "xlstm_narrow_vectors": (_i, [_vp, ctypes.POINTER(_vp), ctypes.POINTER(_vp), ctypes.POINTER(_i), ctypes.POINTER(_f), _i]),
     "xlstm_embedding_scatter_add": (_i, [_vp] * 5 + [_i, _i]),
     "xlstm_split3_bf16": (_i, [_vp] * 5 + [_sz]),
     "xlstm_adamw_multi": (_i, [_vp, ctypes.POINTER(AdamwDesc), _i, _f, _f, _f, _f, _f, _f, _i]),

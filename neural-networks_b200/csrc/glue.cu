@@ -581,3 +581,36 @@ extern "C" int xlstm_bias_rows(void* stream, const float* residual, const float*
     XL_LAUNCH_OK("bias_rows");
     return XLSTM_OK;
 }
+
+// A few thousand values a vector: the launch is what it costs, so a cell's vectors share one.
+namespace xl {
+struct NarrowVectors {
+    const float* x[8];
+    bf16* out[8];
+    int n[8];
+    float scale[8];
+};
+static __global__ void __launch_bounds__(256) narrow_vectors_k(const NarrowVectors p) {
+    const float* x = p.x[blockIdx.y];
+    bf16* out = p.out[blockIdx.y];
+    const int n = p.n[blockIdx.y];
+    const float s = p.scale[blockIdx.y];
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) out[i] = __float2bfloat16_rn(s * x[i]);
+}
+}  // namespace xl
+
+extern "C" int xlstm_narrow_vectors(void* stream, const float* const* x, void* const* out_bf16, const int* n, const float* scale, int count) {
+    XL_CHECK_ARG(x && out_bf16 && n && scale && count >= 0 && count <= 8, "narrow_vectors: null pointer or more than eight vectors");
+    NarrowVectors p = {};
+    int most = 0;
+    for (int i = 0; i < count; ++i) {
+        XL_CHECK_ARG(n[i] == 0 || (n[i] > 0 && x[i] && out_bf16[i]), "narrow_vectors: vector %d", i);
+        p.x[i] = x[i]; p.out[i] = (bf16*)out_bf16[i]; p.n[i] = n[i]; p.scale[i] = scale[i];
+        if (n[i] > most) most = n[i];
+    }
+    if (!most) return XLSTM_OK;
+    const int blocks = (most + 255) / 256;
+    narrow_vectors_k<<<dim3(blocks < 1024 ? blocks : 1024, count), 256, 0, (cudaStream_t)stream>>>(p);
+    XL_LAUNCH_OK("narrow_vectors");
+    return XLSTM_OK;
+}

@@ -10,6 +10,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <pybind11/stl.h>
+
 #include <cmath>
 
 #include "../../include/xlstm_b200.h"
@@ -190,20 +192,37 @@ static void embedding_scatter_add(const Tensor& table_g, const Tensor& ids, cons
 
 // ---- projections: Y = X W + b --------------------------------------------------------------------------------------------------------
 // mode 0: fp32 result with the bias; 1: the product alone, fp32; 2: residual + the product + bias (the seed is one pass, the product
-// accumulates into it); 3: scale * (x W + b) rounded once to bf16; 4: the product alone as bf16.
-static Tensor linear_fw(const Tensor& x, const Tensor& w, const Tensor& b, int mode, const OptT& residual, double scale) {
+// accumulates into it); 3: scale * (x W + b) rounded once to bf16, with the bias as narrow_biases leaves it; 4: the product alone as bf16.
+static bool power_of_two(double s) {
+    int e;
+    return std::frexp(s, &e) == 0.5;
+}
+// The biases of a cell's narrowed projections in the operand type, from the fp32 ones at every forward call: a program may have written them
+// since the last. With a factor on the bias too, the library spreads it over the whole output first and reads that back (32768 x 2048:
+// 176 us); a power of two goes into the bias here, which changes no bit.
+static std::vector<Tensor> narrow_biases(const std::vector<Tensor>& b, const std::vector<double>& scale) {
+    Below guard;
+    if (b.size() > 8 || b.size() != scale.size()) refuse("narrow_biases: at most eight, a scale each");
+    const float* x[8];
+    void* out[8];
+    int n[8];
+    float s[8];
+    std::vector<Tensor> r;
+    for (size_t i = 0; i < b.size(); ++i) {
+        r.push_back(fresh(b[i].sizes(), at::kBFloat16, b[i]));
+        x[i] = fptr(b[i]); out[i] = ptr(r[i]); n[i] = (int)b[i].numel();
+        s[i] = power_of_two(scale[i]) ? (float)scale[i] : 1.f;
+    }
+    check(xlstm_narrow_vectors(stream(), x, out, n, s, (int)b.size()), "narrow_biases");
+    return r;
+}
+static Tensor linear_fw(const Tensor& x, const Tensor& w, const Tensor& b, const OptT& narrowed, int mode, const OptT& residual, double scale) {
     Below guard;
     const bool bf = w.scalar_type() == at::kBFloat16;
     if (mode == 4) return at::mm(x, w);
     if (mode == 3) {
-        // the bias in the operand type, from the fp32 one at every call: a program may have written it since the last
-        // with a factor on the bias too, the library spreads it over the whole output first and reads that back (32768 x 2048: 176 us); a power
-        // of two can go into the bias beforehand without changing a bit
-        int e;
-        if (scale == 1.0 || std::frexp(scale, &e) != 0.5) return at::addmm(b.to(at::kBFloat16), x, w, scale, scale);
-        Tensor sb = fresh(b.sizes(), at::kBFloat16, b);
-        at::mul_out(sb, b, at::scalar_tensor(scale, at::kDouble));
-        return at::addmm(sb, x, w, 1, scale);
+        const Tensor nb = narrowed ? *narrowed : narrow_biases({b}, {scale})[0];
+        return at::addmm(nb, x, w, power_of_two(scale) ? 1.0 : scale, scale);
     }
     if (mode == 2) {
         Tensor out = bias_rows(b, residual->size(0), residual);
@@ -314,6 +333,7 @@ PYBIND11_MODULE(_host, m) {
     m.def("ogate_fw", &ogate_fw);
     m.def("ogate_bw", &ogate_bw);
     m.def("embedding_scatter_add", &embedding_scatter_add);
+    m.def("narrow_biases", &narrow_biases);
     m.def("linear_fw", &linear_fw);
     m.def("linear_bw", &linear_bw);
     m.def("adamw", &adamw);

@@ -82,17 +82,18 @@ class Linear:
         self.w = Param(w, decay, shadow=bf16)
         self.b = Param(b, False)
 
-    def forward(self, x, bias=True, residual=None, narrow=False, scale=1.0):
+    def forward(self, x, bias=True, residual=None, narrow=False, scale=1.0, narrowed=None):
         """x: fp32, or already narrowed to bf16 by a caller that feeds several projections from it.
         bias=False: the product alone (the consumer kernel adds the bias). residual: returns residual + x W + b,
         with one pass that seeds the output with residual + b and the product accumulated inside the GEMM (the
         reference's broadcast_row_resid seed, src/gpu/cuda/common.cu:20-48). narrow (bf16 layers): the result
-        straight from the GEMM epilogue as bf16, scale * (x W + b), rounded once."""
+        straight from the GEMM epilogue as bf16, scale * (x W + b), rounded once; `narrowed`: this call's
+        ops.narrow_biases of it, where several projections share one."""
         self.x = _b16(x) if self.bf16 else x
         narrow = narrow and self.bf16
         assert scale == 1.0 or (narrow and bias), "scale is folded only into the narrowed epilogue"
         mode = (3 if bias else 4) if narrow else 2 if residual is not None else 0 if bias else 1
-        return ops.linear_forward(self.x, self.w.wb if self.bf16 else self.w.w, self.b.w, mode, residual, scale)
+        return ops.linear_forward(self.x, self.w.wb if self.bf16 else self.w.w, self.b.w, narrowed, mode, residual, scale)
 
     def backward(self, dy, need_dx=True, accum=None, scale=1.0, narrow_dx=False):
         """Accumulates dW, db; returns dx, added into `accum` (inside the GEMM, beta = 1) when one is given.
@@ -167,9 +168,10 @@ class MLstm:
         if self.bf16:
             x = _b16(x)  # one narrowing feeds all six projections
         if self.bf16:  # bf16 q, k, v straight from the GEMM epilogue (bias and the 1/sqrt(dqk) of k folded in)
-            q = self.lq.forward(x, narrow=True)
-            k = self.lk.forward(x, narrow=True, scale=self.inv_sqrt)
-            v = self.lv.forward(x, narrow=True)
+            bq, bk, bv = ops.narrow_biases([self.lq.b.w, self.lk.b.w, self.lv.b.w], [1.0, self.inv_sqrt, 1.0])
+            q = self.lq.forward(x, narrow=True, narrowed=bq)
+            k = self.lk.forward(x, narrow=True, scale=self.inv_sqrt, narrowed=bk)
+            v = self.lv.forward(x, narrow=True, narrowed=bv)
         else:
             q = self.lq.forward(x)
             k = self.lk.forward(x).mul_(self.inv_sqrt)

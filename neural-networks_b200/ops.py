@@ -245,7 +245,9 @@ def ogate_backward(d_hc, o, yhat, out_dtype=torch.float32):
     return host.ogate_bw(d_hc, o, yhat, out_dtype == torch.bfloat16)
 
 
-# A projection with its library GEMMs (layers.Linear): see linear_fw / linear_bw of csrc_host/host.cpp for the modes.
+# A projection with its library GEMMs (layers.Linear): see linear_fw / linear_bw of csrc_host/host.cpp for the modes, and the biases of
+# several narrowed ones.
+narrow_biases = timed("narrow_biases")(host.narrow_biases)
 linear_forward = timed("projection_forward")(host.linear_fw)
 linear_backward = timed("projection_backward")(host.linear_bw)
 
