@@ -84,8 +84,8 @@ def test_mlstm_full_size_sample_against_oracle_carry_and_linearity(B, H, T, d, h
 
 @pytest.mark.parametrize("B,H,NH,T", [(32, 1024, 4, 1024), (8, 2048, 4, 1024)])
 def test_slstm_full_size_sample_against_oracle_and_carry(B, H, NH, T):
-    """configs[2] (B32, 4 x 256, S1024) on the cluster kernels and the sLSTM layer of configs[3] (B8, 4 x 512; the
-    sequence cut to 1024 positions to bound the oracle's time) on the grid kernels; fp32."""
+    """32 sequences of 4 x 256 units over 1024 positions and the language model's sLSTM layer (8 of 4 x 512; the sequence cut to
+    1024 positions to bound the oracle's time), both on the register-resident loops; fp32."""
     from gpu_util import ops, xl
     dh = H // NH
     wh = _gen((NH, dh, 4 * dh), 11, scale=dh ** -0.5)
