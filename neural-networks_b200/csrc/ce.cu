@@ -275,7 +275,10 @@ __global__ void __launch_bounds__(256) ce_tile(const float* logits, const uint32
         float* tile = tiles + s * stage;
         const bool ok = tc::mbar_wait(full + s, (k / kCeStages) & 1);
         if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicCAS(status, 0, 401);
+            if (tid == 0) {
+                atomicCAS(status, 0, 401);
+                if (t + (int)gridDim.x < ntiles) (void)tc::mbar_wait(full + (k + 1) % kCeStages, ((k + 1) / kCeStages) & 1);  // the next tile's load is on its way
+            }
             break;
         }
         if (n != whole) {

@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) par_grad(const __grid_constan
                 pair(i++, &p.tq, t0, x + 2 * f, b);   // dS^T Q; kept for dq.q
                 pair(i++, &p.tdn, t0, x + 2 * f, b);  // DS^T dN
             }
+            if (fail) ring_landed<R>(full, n);
         }
         __syncwarp();
     } else if (warp == 17) {

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kOutThreads, 1) par_out(const __grid_constant_
                 }
                 pair(&p.tv, t0, x + 2 * f, b);
             }
+            if (fail) ring_landed<OutS::R>(full, n);
         }
         __syncwarp();
     } else if (warp == 17) {

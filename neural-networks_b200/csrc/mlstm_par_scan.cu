@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
     if (warp == 16) {
         // ---- loads ----
         if (lane == 0) {
-            for (int i = 0; i < halves && !fail; ++i) {
+            int i = 0;
+            for (; i < halves && !fail; ++i) {
                 const int st = i % S::kStages, ck = chunk(i >> 1), t0 = ck * LC + (i & 1) * 64;
                 if (i >= S::kStages) PAR_WAIT(empty + st, ((i / S::kStages) - 1) & 1);
                 if (fail) break;
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) par_scan(const __grid_constan
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 256, [%2];"
                              ::"r"(smem_u32(sw + st * 64)), "l"(p.w + (size_t)bh * p.Tp + t0), "r"(smem_u32(full + st)) : "memory");
             }
+            if (fail) ring_landed<S::kStages>(full, i);
         }
         __syncwarp();
     } else if (warp == 17) {
